@@ -121,15 +121,21 @@ static __device__ bool live_path(const WaveGroups& G, int cur, uint32_t k, LiveP
     return false;
 }
 
-// cur < 0: the whole render, its first camera rays made by k_paths_init; else what the bounce loop left,
-// the live paths of parity cur (at most kPathSlots per block).
+// cur_queues < 0: the whole render, its first camera rays made by k_paths_init; else what the bounce loop
+// left, the live paths of parity cur_queues.  With more than `most` of those the loop did not hand over: its
+// cap ended it, the render is an error, and nothing is run.
 template <int THREADS, bool GENERAL, int ADJ>
 __global__ void __launch_bounds__(THREADS, 1)
     k_wave_paths(const __grid_constant__ WaveGroups G, DevScene S, DevView V, DevParams P, DevAovs out, int cur_queues,
-                 uint32_t grain_log2, uint32_t* err, uint32_t* progress, const AdjPass* A) {
+                 uint32_t most, uint32_t grain_log2, uint32_t* err, uint32_t* progress, const AdjPass* A) {
     __shared__ BlockQueues q;
     const WaveState& W = G.W[0];  // (groups differ in their queues only)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (cur_queues >= 0) {  // (this kernel leaves these counts alone: every block reads the same)
+        uint32_t handed = 0;
+        for (int g = 0; g < G.groups; ++g) handed += wave_live(G.W[g].counts, cur_queues, G.W[g].defer_cap);
+        if (handed > most) return;
+    }
     if (tid < 2 * kKinds) (&q.n_ready[0][0])[tid] = 0;
     if (tid == 0) q.n_ray = q.n_shadow = q.live = q.active = 0;
     __syncthreads();
@@ -142,7 +148,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (uint32_t base = 0; base < kPathSlots; base += THREADS) {
         const uint32_t l = base + tid, k = dealt(l, grain_log2);
         LivePath p{k, 0, true, true};
-        const bool valid = cur_queues < 0 ? k < W.slots && W.ev_mark[k] : live_path(G, cur_queues, k, p);
+        // (kPathSlots is no multiple of 384 threads)
+        const bool valid = l < kPathSlots && (cur_queues < 0 ? k < W.slots && W.ev_mark[k] : live_path(G, cur_queues, k, p));
         bool shadow = false;
         if (valid) {
             q.slot[l] = p.slot;
@@ -359,8 +366,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 template <int THREADS, bool GENERAL, int ADJ>
 static void launch_paths(const WaveLaunch& L, const WaveGroups& G, int cur, uint32_t grid, uint32_t grain,
                          cudaStream_t st) {
-    k_wave_paths<THREADS, GENERAL, ADJ><<<grid, THREADS, 0, st>>>(G, L.S, L.V, L.P, L.out, cur, grain, L.err, L.progress,
-                                                              L.adj);
+    k_wave_paths<THREADS, GENERAL, ADJ><<<grid, THREADS, 0, st>>>(G, L.S, L.V, L.P, L.out, cur, L.tail_paths, grain,
+                                                              L.err, L.progress, L.adj);
 }
 
 template <int THREADS>

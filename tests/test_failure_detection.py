@@ -65,3 +65,37 @@ def test_traversal_cap_in_trace_and_render(scene, oracle_mod):
     finally:
         g.set_tuning()
     assert np.array_equal(got["object"], want["object"]) and np.array_equal(got["triangle"], want["triangle"])
+
+
+# a cap that stops the loop with more live paths than it hands over, which the path kernel then leaves
+# alone: a launch of its 384-thread form (tail_paths up to 768 a block) and one of its 512-thread form, the
+# general kernels, an adjoint replay's loop, a batch's graph
+@pytest.mark.parametrize("make,w,h,divisor", [(synth.config_c1, 1024, 768, 0), (synth.config_c1, 1024, 768, 1),
+                                              (synth.config_c1, 1920, 1080, 32), (synth.config_features, 1024, 768, 0),
+                                              (synth.config_c1, 64, 48, 0)])
+def test_bounce_loop_cap_of_large_images(gpu_ctx, make, w, h, divisor):
+    torch = pytest.importorskip("torch")
+    from sharpray_gb300 import render_batch, render_params
+    from sharpray_gb300.autograd import current_stream_handle, device_aovs
+    d = make(w, h, 4)
+    d.min_samples = 4  # no pixel is done after two bounces
+    g = d.instantiate(gpu_ctx)
+    g.build()
+    bufs, aovs = device_aovs(w, h)
+    for mode in (_abi.SR_RENDER_WAVEFRONT_GRAPH, _abi.SR_RENDER_AUTO):
+        g.set_render_mode(mode)
+        g.set_tuning(tail_divisor=divisor)
+        before = render(d, g)
+        g.set_tuning(tail_divisor=divisor, max_bounce_iterations=2)
+        with pytest.raises(SharpRayError) as e:
+            render(d, g)
+        assert e.value.code == _abi.SR_ERR_DEVICE and "loop cap" in str(e.value)
+        render_batch([g], [d.view], [render_params(*d.render_args())], [aovs], current_stream_handle())
+        torch.cuda.synchronize()
+        with pytest.raises(SharpRayError) as e:  # the batch's error word, read by the next synchronous call
+            g.trace(seeded_rays(8, seed=1))
+        assert "loop cap" in str(e.value)
+        g.set_tuning(tail_divisor=divisor)
+        after = render(d, g)
+        for plane in ("radiance", "radiance_fog", "samples", "depth"):
+            assert np.array_equal(getattr(before, plane).view(np.uint32), getattr(after, plane).view(np.uint32)), plane
