@@ -475,13 +475,6 @@ struct Hit {
 // prunes nothing, which gives the same yes/no answer as the closest-hit query.
 constexpr int kSceneStack = 192;  // scene (<= 65) + mesh (<= 65) entries, with margin
 
-// How far a search goes that needs the hits up to `dist` only: 1 % and 1e-4 of the origin's coordinates
-// further, thousands of roundings more than what a box's or a triangle's distance can be off by, so that
-// everything up to `dist` is found as in a full search.  A NaN sets no limit.
-SR_DEV float search_limit(float dist, const Ray& r) {
-    return fminf(1.01f * dist + 1e-4f * (fabsf(r.o.x) + fabsf(r.o.y) + fabsf(r.o.z)), __int_as_float(0x7f800000));
-}
-
 // Resumable traversal state.  init() starts a ray; the query is then a sequence of actions, each
 // chosen by `state`:
 //   QS_NODE : visit the next node -- the nearer child kept from the last visit (the reference
@@ -570,10 +563,6 @@ struct SceneQuery {
             state = QS_NODE;
         }
     }
-
-    // Hits beyond `dist` need not be found (a ray that scatters in fog there): the query may then end
-    // without a hit.
-    SR_DEV void limit(float dist) { best.dist = cur_best = search_limit(dist, wr); }
 
     // The action after the current one, in the reference's order: finish the current mesh, then
     // the remaining objects of the current scene leaf, then the stack.
@@ -699,10 +688,14 @@ struct SceneQuery {
                     in_mesh = true;
                     cr = l;
                     // A hit behind the one the ray already has changes nothing, so it need not be looked
-                    // for (work-counting queries do, as the reference does).  A 641x479 render of the
-                    // feature scene's overlapping objects 31.95 -> 30.87 ms, the 1080p fog frame
-                    // 234.35 -> 234.0.
-                    cur_best = COUNT || is_any() ? inf : search_limit(best.dist * lscale, l);
+                    // for (work-counting queries do, as the reference does).  The bound lies 1 % and
+                    // 1e-4 of the origin's coordinates beyond that hit: thousands of roundings more
+                    // than what a box's or a triangle's distance can be off by, so that everything up
+                    // to it is found as in a full search.  A 641x479 render of the feature scene's
+                    // overlapping objects 31.95 -> 30.87 ms, the 1080p fog frame 234.35 -> 234.0.
+                    cur_best = inf;
+                    if (!COUNT && !is_any() && best.obj >= 0)
+                        cur_best = 1.01f * (best.dist * lscale) + 1e-4f * (fabsf(l.o.x) + fabsf(l.o.y) + fabsf(l.o.z));
                     ob_tri = -1;
                 }
             } else if (GENERAL) {
@@ -736,10 +729,10 @@ struct SceneQuery {
 };
 
 // True when a query's first step -- the two children of the scene BVH's root -- already decides it
-// (neither box is hit up to `limit`, so there is no hit), without a traversal; counts what that step
-// counts.  False when the root is a leaf or a child box is hit.
+// (neither box is hit, so there is no hit), without a traversal; counts what that step counts.
+// False when the root is a leaf or a child box is hit.
 template <bool COUNT, bool ANY>
-SR_DEV bool misses_scene(const DevScene& S, const Ray& r, Ctr& c, float limit) {
+SR_DEV bool misses_scene(const DevScene& S, const Ray& r, Ctr& c) {
     if (S.tlas_root < 0) return true;
     const float4* root = S.nodes + 2 * S.tlas_root;
     float4 rn0 = ldg4(root), rn1 = ldg4(root + 1);
@@ -747,9 +740,10 @@ SR_DEV bool misses_scene(const DevScene& S, const Ray& r, Ctr& c, float limit) {
     SR_COUNT(c, SR_COUNTER_TLAS_NODE, 2);
     const float4* n = S.nodes + 2 * __float_as_int(rn0.w);
     float4 a0 = ldg4(n), a1 = ldg4(n + 1), b0 = ldg4(n + 2), b1 = ldg4(n + 3);
+    const float inf = __int_as_float(0x7f800000);
     float ta = 0.f, tb = 0.f;
-    bool pa = slab(a0, a1, r, ta) && (ANY || ta <= limit);
-    bool pb = slab(b0, b1, r, tb) && (ANY || tb <= limit);
+    bool pa = slab(a0, a1, r, ta) && (ANY || ta <= inf);
+    bool pb = slab(b0, b1, r, tb) && (ANY || tb <= inf);
     return !pa && !pb;
 }
 

@@ -179,12 +179,10 @@ __device__ __forceinline__ int segment_event(float fog_t, bool has_hit, float hi
 
 // A new path ray (scatter or camera ray) with fog scatter distance fog_t: -1 when it needs the
 // next trace kernel's traversal; when it misses both root children of the scene BVH -- the first
-// thing the traversal tests -- or scatters before it reaches them, it has no hit that counts, and its
-// segment's event is returned.
+// thing the traversal tests -- it has no hit, and its segment's event is returned.
 template <bool COUNT>
 __device__ __forceinline__ int next_segment(const DevScene& S, const Ray& ray, float fog_t, Ctr& c) {
-    const float limit = COUNT ? __int_as_float(0x7f800000) : search_limit(fog_t, ray);
-    if (!misses_scene<COUNT, false>(S, ray, c, limit)) return -1;
+    if (!misses_scene<COUNT, false>(S, ray, c)) return -1;
     SR_COUNT(c, SR_COUNTER_SCENE_TRACE, 1);
     return segment_event(fog_t, false, 0.f);
 }
@@ -339,9 +337,7 @@ struct LaneQueries : LaneAll {
 // distance) stores its answer and returns an output code that `emit(slot, code)` (all lanes
 // together, -1 = none) passes on.  Shadow rays are occlusion queries, or with ANY_HIT = false (scenes
 // with transparent objects) closest-hit queries like the path rays: finish may then return kGoOn with
-// `ray` the next ray of the same entry.  LIMITED: a path ray's hits beyond its scatter distance change
-// nothing and are not looked for (the 1080p fog frame 232.4 -> 230.5 ms; with rays that scatter before
-// the scene's root boxes answered at once, next_segment, a 641x479 feature scene 30.5 -> 30.1 ms).
+// `ray` the next ray of the same entry.
 // Each round runs the node visits of all lanes together (up to kNodeBurst), then one leaf action
 // of each lane that waits for one: leaf actions are long and differ between lanes, so batching
 // them keeps warps from running each one with a single lane.  Finished lanes are answered in a
@@ -365,8 +361,8 @@ constexpr int kDeferF4 = kDeferHeadF4 + (3 * kSceneStack + 3) / 4;
 static_assert(kDeferF4 * sizeof(float4) == kDeferBytes, "host and device sizes of a defer record differ");
 
 constexpr int kGoOn = -2;
-template <bool COUNT, bool GENERAL, typename Lanes = LaneAll, bool ANY_HIT = true, bool LIMITED = false,
-          typename Start, typename Finish, typename Emit>
+template <bool COUNT, bool GENERAL, typename Lanes = LaneAll, bool ANY_HIT = true, typename Start, typename Finish,
+          typename Emit>
 __device__ __forceinline__ void persistent_queries(const DevScene& S, const Rec* q0, uint32_t n0, const Rec* q1,
                                                    uint32_t n1, uint32_t* fetch, Ctr& c, uint32_t* err, Start start,
                                                    Finish finish, Emit emit, const float4* din = nullptr,
@@ -441,7 +437,6 @@ __device__ __forceinline__ void persistent_queries(const DevScene& S, const Rec*
                     start(any);
                     shadow = any;
                     sq.init(S, make_ray(V3{e.a.x, e.a.y, e.a.z}, V3{e.b.x, e.b.y, e.b.z}), ANY_HIT && any);
-                    if (LIMITED && !COUNT && !any) sq.limit(__uint_as_float(tag));
                     busy = true;
                 }
             }
@@ -563,7 +558,7 @@ __global__ void __launch_bounds__(BLOCK, (LOOP_SHADOWS ? SR_TRACE_LOOP_BLOCKS : 
 #pragma unroll
     for (int i = 0; i < SR_COUNTER_COUNT; ++i) c.v[i] = 0;
     [[maybe_unused]] ShadowChain chain;
-    persistent_queries<COUNT, GENERAL, LaneAll, !LOOP_SHADOWS, true>(
+    persistent_queries<COUNT, GENERAL, LaneAll, !LOOP_SHADOWS>(
         S, W.q_trace[cur], W.counts[kCountTrace + cur], W.q_shadow[cur], W.counts[kCountShadow + cur],
         &W.counts[kCountTraceFetch], c, err,
         [&](bool any) {
@@ -791,8 +786,7 @@ __device__ __forceinline__ SegOut shade_event(const WaveState& W, const DevScene
                 const bool to_fog = fog_event && bounce == 0;
                 Ray shadow = make_ray(pos, ldir);
                 const bool any = !GENERAL || !S.has_transparent;
-                const float inf = __int_as_float(0x7f800000);
-                if (any ? misses_scene<COUNT, true>(S, shadow, c, inf) : misses_scene<COUNT, false>(S, shadow, c, inf)) {
+                if (any ? misses_scene<COUNT, true>(S, shadow, c) : misses_scene<COUNT, false>(S, shadow, c)) {
                     // a shadow ray that misses the scene's root boxes is unoccluded: its
                     // transmittance is the fog's alone, and the light sample's contribution is
                     // added at once, as SampleSkyDirect(Fog) forms it

@@ -318,7 +318,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                             const Rec r = ld_rec(&W.rec[rix(W, s, any ? R_SH0 : R_RAY)]);
                             sq.init(S, make_ray(V3{r.a.x, r.a.y, r.a.z}, V3{r.b.x, r.b.y, r.b.z}),
                                     any && !loop_shadows);
-                            if (!any) sq.limit(r.b.w);
                             if (loop_shadows && any) chain.begin();
                             shadow = any;
                             busy = true;
