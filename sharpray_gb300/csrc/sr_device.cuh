@@ -687,15 +687,7 @@ struct SceneQuery {
                     has_node = true;
                     in_mesh = true;
                     cr = l;
-                    // A hit behind the one the ray already has changes nothing, so it need not be looked
-                    // for (work-counting queries do, as the reference does).  The bound lies 1 % and
-                    // 1e-4 of the origin's coordinates beyond that hit: thousands of roundings more
-                    // than what a box's or a triangle's distance can be off by, so that everything up
-                    // to it is found as in a full search.  A 641x479 render of the feature scene's
-                    // overlapping objects 31.95 -> 30.87 ms, the 1080p fog frame 234.35 -> 234.0.
                     cur_best = inf;
-                    if (!COUNT && !is_any() && best.obj >= 0)
-                        cur_best = 1.01f * (best.dist * lscale) + 1e-4f * (fabsf(l.o.x) + fabsf(l.o.y) + fabsf(l.o.z));
                     ob_tri = -1;
                 }
             } else if (GENERAL) {

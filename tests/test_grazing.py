@@ -53,3 +53,36 @@ def test_grazing_hits_in_fog(gpu_ctx, length, density, seed):
         assert 0 < np.isfinite(want["depth"]).sum()
         for k in want:
             assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
+
+
+def wall(at, frame, offset):
+    """A quad across the strip's way, and a sliver before the strip that makes its box start first."""
+    c = [(-2.0, -2.0), (2.0, -2.0), (2.0, 2.0), (-2.0, 2.0)]
+    q = np.array([at * frame[0] + y * frame[1] + z * frame[2] for y, z in c])
+    s = np.array([-15.0 * frame[0] + y * frame[1] + z * frame[2] for y, z in ((3.0, 0.5), (3.1, 0.5), (3.0, 0.6))])
+    pos = np.stack([q[[0, 1, 2]], q[[0, 2, 3]], s]) + offset
+    return synth.MeshDesc(pos.astype(np.float32), np.zeros((3, 3, 2), np.float32))
+
+
+@pytest.mark.parametrize("length", [8.0, 80.0, 800.0])
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_grazing_hits_behind_a_wall(gpu_ctx, oracle_mod, length, seed):
+    """Rays that already have a hit, on a wall, find the strip's hits before it as the oracle does."""
+    d, rng, frame, offset = strip_scene(seed, length)
+    d.meshes.append(wall(0.3 * length, frame, offset))
+    d.objects.append(synth.ObjectDesc("wall", synth.Transform(), d.objects[0].material, ("mesh", 1)))
+    n = 20000
+    o = -20.0 * frame[0] + rng.uniform(-0.5, 0.5, (n, 1)) * frame[1] + offset
+    way = length * frame[0] + rng.uniform(-1.0, 1.0, (n, 1)) * frame[1] + offset - o
+    rays = np.concatenate([o, way / np.linalg.norm(way, axis=1, keepdims=True)], axis=1).astype(np.float32)
+    g = d.instantiate(gpu_ctx)
+    g.build()
+    want = oracle_mod.instantiate(d).trace(rays)
+    assert (want["object"] == 0).sum() > 1000 < (want["object"] == 1).sum()
+    for mode in (_abi.SR_RENDER_AUTO, _abi.SR_RENDER_MEGAKERNEL):
+        g.set_render_mode(mode)
+        got = g.trace(rays)
+        for k in ("object", "triangle"):
+            assert np.array_equal(got[k], want[k]), k
+        for k in ("dist", "uv"):
+            assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
