@@ -88,6 +88,17 @@ void wave_adj_grid_sizes(WaveLaunch& L, int sms) {
     L.grid_adj_finalize = sms * (fin > 0 ? fin : 1);
 }
 
+// The caller's float takes the whole sum at once: added to it sample by sample, in float, 300,000 samples
+// came out 3e-6 off and 2.4 million 8e-6, differently in each run.
+__global__ void k_adj_density(const AdjPass* A) {
+    if (*A->density != 0.0) atomicAdd(A->grad_f, (float)*A->density);
+}
+
+cudaError_t wave_adj_density(const AdjPass* pass, cudaStream_t st) {
+    k_adj_density<<<1, 1, 0, st>>>(pass);
+    return cudaGetLastError();
+}
+
 // Record mode's sweep: one thread per (slot, kept sample) -- every slot of every group, its pixel
 // from the 8x4 tile layout -- over the samples the pixel took, with G = dL/dI / its sample count.
 __global__ void __launch_bounds__(128) k_adjoint_checkpoint(WaveState W, DevScene S, DevParams P, const AdjPass* A,

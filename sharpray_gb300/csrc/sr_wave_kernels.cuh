@@ -1193,14 +1193,16 @@ __global__ void __launch_bounds__(128) k_wave_finalize(WaveState W, DevScene S, 
     const uint32_t n = LATE ? W.counts[kCountLate + cur] : W.counts[count_resolve(cur)];
     const uint32_t* q = LATE ? W.q_late[cur] : W.q_resolve[cur];
     const uint32_t stride = gridDim.x * blockDim.x;
-    float g_density = 0.0f;  // adjoint replay: this thread's d loss / d fog density
+    [[maybe_unused]] double g_density = 0.0;  // adjoint replay: this thread's d loss / d fog density
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         uint32_t k = base + threadIdx.x;
         bool valid = k < n;
         uint32_t s = valid ? q[k] : 0u;
         SegOut o;
         if (valid) {
-            o = finalize_sample<COUNT, GENERAL, ADJ>(W, S, V, P, out, s, c, A, &g_density);
+            float g = 0.0f;
+            o = finalize_sample<COUNT, GENERAL, ADJ>(W, S, V, P, out, s, c, A, &g);
+            if constexpr (ADJ == kAdjReplay) g_density += (double)g;
         }
         uint32_t* eq = W.q_event[nxt];
         const bool pred[3] = {valid && o.live && o.next < 0, valid && o.live && o.next == EV_FOG,
@@ -1216,7 +1218,7 @@ __global__ void __launch_bounds__(128) k_wave_finalize(WaveState W, DevScene S, 
     flush_counters<COUNT>(c, counters);
     if constexpr (ADJ == kAdjReplay) {  // every thread of the block gets here: one atomic per warp
         for (int d = 16; d > 0; d >>= 1) g_density += __shfl_xor_sync(0xffffffffu, g_density, d);
-        if ((threadIdx.x & 31) == 0 && A->grad_f && g_density != 0.0f) atomicAdd(A->grad_f, g_density);
+        if ((threadIdx.x & 31) == 0 && A->grad_f && g_density != 0.0) atomicAdd(A->density, g_density);
     }
 }
 

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     __syncthreads();
 
     Ctr c;
-    double g_density = 0.0;
+    [[maybe_unused]] double g_density = 0.0;  // adjoint replay: this thread's d loss / d fog density
     const bool loop_shadows = GENERAL && S.has_transparent;
 
     // ---- the block's paths ----
@@ -153,7 +153,6 @@ __global__ void __launch_bounds__(THREADS, 1)
         bool shadow = false;
         if (valid) {
             q.slot[l] = p.slot;
-            if (ADJ == kAdjReplay && cur_queues >= 0) W.medium[p.slot].x = 0.0f;
             shadow = !p.traced && (ibits(ld_rec(&W.rec[rix(W, p.slot, R_PATH)]).b.w) & PF_NEE);
             q.word[l] = ((uint32_t)p.then << 8) | ((p.ray ? 1u : 0u) + (shadow ? 1u : 0u));
         }
@@ -211,19 +210,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t s = q.slot[l];
                 SegOut o;
                 if (kind == K_FIN) {
-                    // adjoint replay: d loss / d fog density, summed in double over what the block runs, or
-                    // over all that a slot was handed over with (in the slot's medium word, which replays
-                    // do not use) as a thread per slot would
-                    float g = ADJ == kAdjReplay && cur_queues >= 0 && valid ? W.medium[s].x : 0.0f;
+                    float g = 0.0f;
                     if (valid) o = finalize_sample<false, GENERAL, ADJ>(W, S, V, P, out, s, c, A, &g);
-                    if constexpr (ADJ == kAdjReplay) {
-                        if (cur_queues < 0)
-                            g_density += (double)g;
-                        else if (valid && o.live)
-                            W.medium[s].x = g;
-                        else if (valid && A->grad_f && g != 0.0f)
-                            atomicAdd(A->grad_f, g);
-                    }
+                    if constexpr (ADJ == kAdjReplay) g_density += (double)g;
                     const unsigned dead = __ballot_sync(0xffffffffu, valid && !o.live);
                     if (lane == 0 && dead) atomicSub(&q.live, (uint32_t)__popc(dead));
                 } else if (valid) {
@@ -349,14 +338,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (busy) sq.save(carried);
         }
     }
-    if constexpr (ADJ == kAdjReplay) {  // one atomic addition per block: each rounds the whole sum so far
+    if constexpr (ADJ == kAdjReplay) {
         __shared__ double part[THREADS / 32];
         for (int d = 16; d > 0; d >>= 1) g_density += __shfl_xor_sync(0xffffffffu, g_density, d);
         if (lane == 0) part[warp] = g_density;
         __syncthreads();
         if (tid == 0 && A->grad_f) {
             for (int w = 1; w < THREADS / 32; ++w) g_density += part[w];
-            if (g_density != 0.0) atomicAdd(A->grad_f, (float)g_density);
+            if (g_density != 0.0) atomicAdd(A->density, g_density);
         }
     }
 }

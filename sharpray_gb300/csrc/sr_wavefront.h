@@ -166,6 +166,7 @@ struct AdjPass {
     float* grad_a;                // dL/d(albedo texels), texture w x h x 3
     float* grad_r;                // dL/d(roughness texels), texture w x h x 3 (channel 0)
     float* grad_f;                // dL/d(fog density), one float
+    double* density;              // replay: what this pass adds to it
 };
 
 struct WaveLaunch {
@@ -279,6 +280,8 @@ void wave_adj_finalize(const WaveLaunch& L, const WaveState& W, int cur, cudaStr
 // `events`: bit 0 fog, bit 1 miss, bit 2 surface (phase 0 never has surface events).
 void wave_adj_shade(const WaveLaunch& L, const WaveState& W, int cur, int phase, cudaStream_t st, int events = 7);
 void wave_adj_grid_sizes(WaveLaunch& L, int sms);
+// After a replay that sums the fog density's gradient: the sum added to the caller's float.
+cudaError_t wave_adj_density(const AdjPass* pass, cudaStream_t st);
 // The whole render (or adjoint pass) as one persistent kernel, without bounces (sr_wave_paths.cu); the
 // camera rays are drawn from random-number stream `seed`.  In place of wave_init, the loop and the tail.
 cudaError_t wave_paths(const WaveLaunch& L, uint32_t seed, int sms, cudaStream_t st);

@@ -503,3 +503,31 @@ def test_checkpointed_adjoint_equals_replay(torch_mod, fog):
     rig.scene.release_checkpoint()
     with pytest.raises(StateError):
         rig.scene.adjoint_checkpointed(d_image.data_ptr(), ta, g[0].data_ptr())
+
+
+# replays by the path kernel and by the bounce loop with its hand-over, with as many samples and with more
+# than a float can be added to one by one
+@pytest.mark.parametrize("mode", [_abi.SR_RENDER_AUTO, _abi.SR_RENDER_WAVEFRONT_GRAPH, _abi.SR_RENDER_WAVEFRONT])
+@pytest.mark.parametrize("w,h,spp", [(40, 30, 4), (192, 192, 8), (200, 200, 8), (384, 384, 16), (640, 512, 8)])
+def test_density_gradient_sums_exactly(torch_mod, mode, w, h, spp):
+    """The replay is linear in dL/dI, so the density gradients of disjoint parts of the image add up to the
+    whole image's, and every part's samples are the same floats in both.  A sum that rounds once per call is
+    then within 2^-24 of the parts' magnitudes, and another 2^-24 of its own, of their sum."""
+    torch = torch_mod
+    d = roughness_scene(spp)
+    d.width, d.height, d.bounces = w, h, 6
+    d.fog = Fog(0.08, (0.8, 0.75, 0.7), 0.5, 0.2)
+    rig = Rig(torch, d)
+    rig.scene.set_render_mode(mode)
+    img = rig.image()
+    d_image = torch.from_numpy((2.0 * (img * np.float32(0.4) - np.float32(0.05))).astype(np.float32)).cuda()
+    ta, tr = rig.tex[1], rig.tex[3]
+    whole = float(adjoint_all(rig, d_image, ta, tr, True)[2][0])
+    edges = np.linspace(0, d_image.numel(), 9).astype(int)
+    parts = []
+    for a, b in zip(edges[:-1], edges[1:]):
+        part = torch.zeros_like(d_image)
+        part[a:b] = d_image[a:b]
+        parts.append(float(adjoint_all(rig, part, ta, tr, True)[2][0]))
+    assert abs(whole) > 0.0
+    assert abs(whole - sum(parts)) <= 2.0 ** -24 * (sum(abs(p) for p in parts) + abs(whole)), (whole, parts)
