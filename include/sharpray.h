@@ -404,7 +404,8 @@ SR_API int sr_scene_get_tuning(SrScene* scene, SrTuning* tuning);
  * blocks per SM (all that fit, one or two fewer), fog-shade blocks per SM (all, two fewer), tail
  * hand-over (slots / 8, 16, 32), slot capacity (every pixel, a half, a quarter) -- keeping the
  * fastest of each, and leaves the result on the scene
- * (ms: its trial time; default_ms: the defaults').  The BVH node width is not a dimension: the
+ * (ms: its trial time; default_ms: the defaults').  A render that SR_RENDER_AUTO gives to the path
+ * kernel is tuned in that form, which has the slot capacity only.  The BVH node width is not a dimension: the
  * traversal walks the reference's binary tree, whose child order the bit-exact hits rest on. */
 SR_API int sr_scene_autotune(SrScene* scene, const SrView* view, const SrRenderParams* params, uint32_t trial_spp,
                              SrTuning* chosen);

@@ -212,3 +212,21 @@ def test_hand_over_to_path_kernel(gpu_ctx, make, w, h, slots, divisor):
                                       (features, 304, 384), (features, 304, 388)])
 def test_path_kernel_block_sizes(gpu_ctx, make, w, h):
     test_path_kernel_matches_bounce_loop(gpu_ctx, make, w, h, 2, 1, 4, 0, 1)
+
+
+@pytest.mark.parametrize("w,h,mode,paths", [(96, 64, _abi.SR_RENDER_AUTO, True), (616, 512, _abi.SR_RENDER_AUTO, False),
+                                            (96, 64, _abi.SR_RENDER_WAVEFRONT_GRAPH, False)])
+def test_autotuner_times_the_form_that_runs(gpu_ctx, w, h, mode, paths):
+    from sharpray_gb300 import render_params
+    d = mesh(w, h)
+    g = d.instantiate(gpu_ctx)
+    g.build()
+    g.set_render_mode(mode)
+    chosen = g.autotune(d.view, render_params(*d.render_args()), trial_spp=2)
+    info = g.render_info()  # of the last trial
+    assert (info["bounce_iterations"] == 0) == paths
+    if paths:  # no other dimension is one of the path kernel's
+        assert (chosen["trace_block_threads"], chosen["trace_blocks_per_sm"], chosen["fog_shade_blocks_per_sm"],
+                chosen["tail_divisor"]) == (128, 0, 0, 8)
+    planes(g, d)
+    assert (g.render_info()["bounce_iterations"] == 0) == paths
