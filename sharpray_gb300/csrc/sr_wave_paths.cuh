@@ -59,6 +59,8 @@ struct BlockQueues {
     uint32_t slot[kPathSlots];  // the block's slots: the global slot of each
     uint32_t word[kPathSlots];  // per slot: what follows its rays (event or K_FIN) << 8 | rays in flight
     uint32_t live;             // slots with a pixel
+    uint64_t turns;            // rounds since a sample was last finished
+    bool stuck;
 };
 
 // Place of item i of kind k in its list.
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (handed > most) return;
     }
     if (tid < 2 * kKinds) (&q.n_ready[0][0])[tid] = 0;
-    if (tid == 0) q.n_ray = q.n_shadow = q.live = q.active = 0;
+    if (tid == 0) q.n_ray = q.n_shadow = q.live = q.active = 0, q.turns = 0;
     __syncthreads();
 
     Ctr c;
@@ -171,7 +173,10 @@ __global__ void __launch_bounds__(THREADS, 1)
     [[maybe_unused]] ShadowChain chain;
     uint32_t l = 0;  // ... and its slot
     int cur = 0;
-    // rounds are bounded by the segments of the samples that the block's pixels can take
+    // A round steps a slot or answers a ray, so until a sample is finished there are at most as many rounds
+    // as the slots' samples have steps and rays: a step, a path ray and a shadow ray for each of bounces + 2
+    // segments, and the sample's end.  Samples are bounded by the pixels' max_samples.
+    const uint64_t most_turns = (uint64_t)kPathSlots * (3ull * ((uint64_t)P.bounces + 2u) + 1u);
     for (;;) {
         __syncthreads();
         const uint32_t live = q.live;
@@ -183,8 +188,13 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
         for (int k = 0; k < kKinds; ++k) ready += n[k] = q.n_ready[cur][k];
         const uint32_t nray = q.n_ray, nshadow = q.n_shadow, kept = q.active;
+        if (tid == 0) {
+            q.turns = n[K_FIN] ? 0 : q.turns + 1;
+            // (neither can happen: a live slot waits for something)
+            q.stuck = q.turns > most_turns || !(ready || nray || nshadow || kept);
+        }
         __syncthreads();  // every thread has read the counts, and takes the same branch
-        if (!ready && !nray && !nshadow && !kept) {  // cannot happen: a live slot waits for something
+        if (q.stuck) {
             if (tid == 0) atomicOr(err, SR_DEVERR_LOOP);
             break;
         }
