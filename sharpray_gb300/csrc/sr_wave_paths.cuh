@@ -59,9 +59,11 @@ struct BlockQueues {
     uint32_t slot[kPathSlots];  // the block's slots: the global slot of each
     uint32_t word[kPathSlots];  // per slot: what follows its rays (event or K_FIN) << 8 | rays in flight
     uint32_t live;             // slots with a pixel
-    uint64_t turns;            // rounds since a sample was last finished
-    bool stuck;
+    bool finished;             // a sample was finished since this was last looked at
+    bool publisher;            // this block publishes the render's progress
+    uint64_t idle;             // rounds since a sample was last seen to be finished
 };
+constexpr uint32_t kLookRounds = 16;  // rounds between looks at these three
 
 // Place of item i of kind k in its list.
 __device__ __forceinline__ uint32_t place(int k, uint32_t i) { return k & 1 ? kPathSlots - 1u - i : i; }
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (handed > most) return;
     }
     if (tid < 2 * kKinds) (&q.n_ready[0][0])[tid] = 0;
-    if (tid == 0) q.n_ray = q.n_shadow = q.live = q.active = 0, q.turns = 0;
+    if (tid == 0) q.n_ray = q.n_shadow = q.live = q.active = 0, q.idle = 0, q.finished = q.publisher = false;
     __syncthreads();
 
     Ctr c;
@@ -176,25 +178,34 @@ __global__ void __launch_bounds__(THREADS, 1)
     // A round steps a slot or answers a ray, so until a sample is finished there are at most as many rounds
     // as the slots' samples have steps and rays: a step, a path ray and a shadow ray for each of bounces + 2
     // segments, and the sample's end.  Samples are bounded by the pixels' max_samples.
-    const uint64_t most_turns = (uint64_t)kPathSlots * (3ull * ((uint64_t)P.bounces + 2u) + 1u);
+    const uint64_t most_idle = (uint64_t)kPathSlots * (3ull * ((uint64_t)P.bounces + 2u) + 1u) + 2u * kLookRounds;
+    uint32_t round = 0;
     for (;;) {
         __syncthreads();
         const uint32_t live = q.live;
         if (live == 0) break;
-        if (progress && blockIdx.x == 0 && tid == 0)
-            *(volatile uint32_t*)progress = *(volatile uint32_t*)(W.counts + kCountDone);
         uint32_t n[kKinds];
         uint32_t ready = 0;
 #pragma unroll
         for (int k = 0; k < kKinds; ++k) ready += n[k] = q.n_ready[cur][k];
         const uint32_t nray = q.n_ray, nshadow = q.n_shadow, kept = q.active;
-        if (tid == 0) {
-            q.turns = n[K_FIN] ? 0 : q.turns + 1;
-            // (neither can happen: a live slot waits for something)
-            q.stuck = q.turns > most_turns || !(ready || nray || nshadow || kept);
-        }
         __syncthreads();  // every thread has read the counts, and takes the same branch
-        if (q.stuck) {
+        bool stuck = !ready && !nray && !nshadow && !kept;  // cannot happen: a live slot waits for something
+        if ((round++ & (kLookRounds - 1u)) == 0) {
+            if (tid == 0) {
+                q.idle = q.finished ? 0 : q.idle + kLookRounds;
+                q.finished = false;
+                stuck = stuck || q.idle > most_idle;
+                // finished pixels, published by one block at a time so that they only grow; one that is done
+                // leaves it to the first that asks
+                if (progress) {
+                    if (!q.publisher) q.publisher = atomicCAS(&W.counts[kCountPublisher], 0u, 1u) == 0u;
+                    if (q.publisher) *(volatile uint32_t*)progress = *(volatile uint32_t*)(W.counts + kCountDone);
+                }
+            }
+            stuck = __syncthreads_or(stuck);
+        }
+        if (stuck) {
             if (tid == 0) atomicOr(err, SR_DEVERR_LOOP);
             break;
         }
@@ -225,6 +236,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if constexpr (ADJ == kAdjReplay) g_density += (double)g;
                     const unsigned dead = __ballot_sync(0xffffffffu, valid && !o.live);
                     if (lane == 0 && dead) atomicSub(&q.live, (uint32_t)__popc(dead));
+                    if (lane == 0) q.finished = true;
                 } else if (valid) {
                     if (kind == EV_SURF)
                         o = shade_segment<false, GENERAL, ADJ, false>(W, S, P, s, EV_SURF, c, A);
@@ -347,6 +359,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             if (busy) sq.save(carried);
         }
+    }
+    if (tid == 0 && q.publisher) {
+        __threadfence_system();
+        atomicExch(&W.counts[kCountPublisher], 0u);
     }
     if constexpr (ADJ == kAdjReplay) {
         __shared__ double part[THREADS / 32];

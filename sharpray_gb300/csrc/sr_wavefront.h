@@ -102,7 +102,7 @@ constexpr size_t kDeferBytes = 16 * (10 + (3 * 192 + 3) / 4);
 constexpr bool kSplitPhases = SR_SPLIT_PHASES && SR_SORT_EVENTS;
 
 // Number of 32-bit counters at WaveState::counts, and their layout.
-constexpr int kWaveCounters = 27;
+constexpr int kWaveCounters = 28;
 enum : int {
     kCountResolve = 0,     // samples finished this bounce without a shadow ray to trace (parity 0;
                            // parity 1: kCountResolve1)
@@ -120,6 +120,7 @@ enum : int {
     kCountPixel = 25,      // group 0: next unclaimed pixel of a render with fewer slots than pixels
     kCountSeed = 26,       // group 0, same renders: the random-number stream of the render (the
                            // bounce kernels' parameters stay seed-independent for graph reuse)
+    kCountPublisher = 27,  // group 0: a block of the path kernel publishes the progress (0: none does)
 };
 #if defined(__CUDACC__)
 __host__ __device__

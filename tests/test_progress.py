@@ -65,3 +65,31 @@ def test_progress_of_batched_renders():
     torch.cuda.synchronize()
     for sc, d in zip(scenes, descs):
         assert sc.progress() == (d.width * d.height, d.width * d.height)
+
+
+def test_progress_goes_on_after_the_first_block():
+    """The path kernel's first block owns the leftmost column of 8x4 tiles here, sky that is done at once;
+    the progress goes on with the blocks that are not."""
+    torch = pytest.importorskip("torch")
+    from sharpray_gb300.autograd import current_stream_handle, device_aovs
+    from sharpray_gb300.synth import look_rotation
+    ctx = Context(0)
+    d = synth.config_c2(8 * torch.cuda.get_device_properties(0).multi_processor_count, 64, 256, rings=200, rock_rings=30,
+                        env=(256, 128))
+    cam = (0.0, 0.0, -3.0)
+    d.objects, d.fog = d.objects[:1], None
+    d.view = synth.View(synth.Transform(cam, look_rotation(cam, (0.0, 0.0, 0.0))), 1.2, 0.1)
+    sc = d.instantiate(ctx)
+    sc.build()
+    _bufs, aovs = device_aovs(d.width, d.height)
+    v, p = d.view.to_c(), render_params(*d.render_args())
+    torch.cuda.synchronize()
+    _abi.check(ctx._lib.sr_render_device(sc.handle, C.byref(v), C.byref(p), C.byref(aovs),
+                                         C.c_void_p(current_stream_handle())))
+    seen = []
+    t0 = time.time()
+    while time.time() - t0 < 60 and (not seen or seen[-1] < d.width * d.height):
+        seen.append(sc.progress()[0])
+    assert seen[-1] == d.width * d.height
+    assert all(a <= b for a, b in zip(seen, seen[1:])), "progress must not go backwards"
+    assert any(d.width * d.height // 2 < s < d.width * d.height for s in seen), sorted(set(seen))[-5:]
