@@ -298,7 +298,8 @@ SR_API int sr_render_compose(SrScene* scene, const SrView* view, const SrRenderP
 enum { SR_RENDER_AUTO = 0, SR_RENDER_MEGAKERNEL = 1, SR_RENDER_WAVEFRONT = 2, SR_RENDER_WAVEFRONT_GRAPH = 3 };
 SR_API int sr_scene_set_render_mode(SrScene* scene, int32_t mode);
 /* Kernel launches and wavefront bounce iterations of the last completed render on this scene
- * (synchronises with it).  No reference counterpart. */
+ * (synchronises with it).  No reference counterpart.  A render that ran as one thread per pixel or as the
+ * persistent kernel has no bounce iterations, and a loop's are those up to its hand-over to that kernel. */
 SR_API int sr_scene_render_info(SrScene* scene, uint32_t* kernel_launches, uint32_t* bounce_iterations);
 /* Reads the work counters of the last render on this scene (device counting is enabled by
  * sr_scene_set_counting); counters_out has SR_COUNTER_COUNT entries. */

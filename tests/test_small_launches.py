@@ -230,3 +230,22 @@ def test_autotuner_times_the_form_that_runs(gpu_ctx, w, h, mode, paths):
                 chosen["tail_divisor"]) == (128, 0, 0, 8)
     planes(g, d)
     assert (g.render_info()["bounce_iterations"] == 0) == paths
+
+
+def test_launches_of_counting_renders(gpu_ctx):
+    """A graph render that counts work runs every bounce itself: it has one launch less than its bounces and
+    loop bodies tell of a render that hands over to the path kernel."""
+    d = mesh(96, 64)
+    g = d.instantiate(gpu_ctx)
+    g.build()
+    g.set_render_mode(_abi.SR_RENDER_WAVEFRONT_GRAPH)
+    planes(g, d)
+    plain = g.render_info()
+    k, n = plain["bounce_iterations"], plain["kernel_launches"]
+    per_bounce, rest = divmod(n - 2 - k // 2, k)  # one launch at the start, one at the end, a condition per two bounces
+    assert rest == 0
+    g.set_counting(True)
+    planes(g, d)
+    counted = g.render_info()
+    k = counted["bounce_iterations"]
+    assert counted["kernel_launches"] == 1 + per_bounce * k + k // 2
