@@ -587,16 +587,6 @@ __global__ void __launch_bounds__(BLOCK, (LOOP_SHADOWS ? SR_TRACE_LOOP_BLOCKS : 
     flush_counters<COUNT>(c, counters);
 }
 
-// The transmittance of slot s's shadow ray by the closest-hit loop (ShadowTransmittance,
-// scene.cs:576-600), times the fog transmittance, written over the request's origin.
-template <bool COUNT, bool GENERAL>
-__device__ __forceinline__ void shadow_trace(const WaveState& W, const DevScene& S, uint32_t s, const Ray& shadow,
-                                             Ctr& c, uint32_t* err) {
-    Col tr = shadow_transmittance<COUNT, GENERAL>(S, shadow, c, err);
-    if (max_component(tr) > 0.0f && S.has_fog) tr = tr * fog_transmittance_inf(S, shadow);
-    st4(&W.rec[rix(W, s, R_SH0)].a, make_float4(tr.r, tr.g, tr.b, 0.f));
-}
-
 // ---- path-vertex records of the adjoint passes (ADJ != kAdjNone) ----------------------------------
 // One record of 8 float4 per vertex (the quantities the reverse sweep needs, as adjoint_sweep's
 // AdjVertex holds them, with the light sample kept apart from its shadow-ray transmittance, which
