@@ -249,3 +249,20 @@ def test_launches_of_counting_renders(gpu_ctx):
     counted = g.render_info()
     k = counted["bounce_iterations"]
     assert counted["kernel_launches"] == 1 + per_bounce * k + k // 2
+
+
+# hand-overs of more than 768 paths a block on 152 SMs, which the 512-thread form takes, up to all that its
+# blocks hold (2,048 slots; half of it for the general kernels, with glass, and one tile row more)
+@pytest.mark.parametrize("make,w,h", [(fog, 616, 512), (mesh, 640, 512), (features, 312, 512), (features, 304, 512)])
+@pytest.mark.parametrize("divisor", [1, 2])
+def test_large_hand_overs(gpu_ctx, make, w, h, divisor):
+    d = make(w, h)
+    d.spp, d.min_samples, d.variance_threshold = 3, 1, 0.1
+    g = d.instantiate(gpu_ctx)
+    g.build()
+    g.set_render_mode(_abi.SR_RENDER_MEGAKERNEL)
+    want = planes(g, d)
+    for mode in (_abi.SR_RENDER_WAVEFRONT, _abi.SR_RENDER_WAVEFRONT_GRAPH):
+        g.set_render_mode(mode)
+        g.set_tuning(tail_divisor=divisor)
+        same(planes(g, d), want)
