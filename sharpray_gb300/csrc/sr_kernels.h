@@ -39,9 +39,10 @@ cudaError_t launch_texels_from_rgb(const float* rgb, float4* out, size_t n, cuda
 cudaError_t launch_trace(const DevScene& S, const float* rays, uint32_t n, int32_t* obj, int32_t* tri, float* dist,
                          float* uv, uint32_t* err, cudaStream_t stream);
 
-// Denoise + fog blur + tonemap (sr_compose.cu).  `spatial` holds the (2r+1)^2 surface weights
-// dw-independent exp(-d^2/(2 r^2)) and `fog_spatial` the fog weights strength*exp(...), both
-// evaluated on the host.  `denoise` = false gives Compositor.Preview.
+// Denoise + fog blur + tonemap (sr_compose.cu, which gives the tables' layout).  `pairs` holds the surface
+// weights exp(-d^2/(2 r^2)) of two pixel rows, `row_half` the kernel rows' half-widths and `fog_spatial`
+// the fog weights strength*exp(...), all evaluated on the host.  `denoise` = false gives
+// Compositor.Preview, without tables.
 struct ComposeConsts {
     int32_t tonemapper;
     float exposure;
